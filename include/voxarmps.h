@@ -198,9 +198,11 @@ int mps_dcg_finish(mps_ctx* ctx, int iters, double relres, double bb);
 
 /* Per-stage device timing with CUDA events (off by default).  While on,
  * scalars ms_neighbors ms_explicit ms_ppe ms_post ms_step (last step) and
- * spmv_ms / spmv_launches, lists_ms (accumulated) are available.  On scenes
- * whose pressure solve is one launch (up to 300,000 particles; 524,288 in mixed
- * precision) spmv_ms is that launch's time and spmv_launches its iterations. */
+ * spmv_ms / spmv_launches, lists_ms (accumulated) are available.  A profiled
+ * FP64 solve takes one launch per kernel at every size (the same bits as in one
+ * launch), and spmv_ms is the products' time.  A mixed-precision solve that is
+ * one launch (up to 524,288 particles, Newtonian fluids) stays so: spmv_ms is
+ * that launch's time and spmv_launches its iterations. */
 int mps_set_profile(mps_ctx* ctx, int on);
 
 /* Graph mode (no reference counterpart; the reference launches every stage

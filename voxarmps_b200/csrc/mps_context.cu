@@ -319,6 +319,7 @@ int allocate(mps_ctx* c)
         TRY(dalloc(c, &c->PH32, P));
     }
     TRY(dalloc(c, &c->PH, P));
+    if (c->cfg.precision == 0 && c->n <= kFormMax) TRY(dalloc(c, &c->cg_zp, P));
     // the cell counts of both grids and len_max: one area, zeroed at once
     TRY(dalloc(c, &c->cnt_l, (size_t)c->gl.tnc + c->gs.tnc + 6));
     c->cnt_s = c->cnt_l + (c->gl.tnc + 2);

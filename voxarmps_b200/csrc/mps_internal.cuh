@@ -35,6 +35,11 @@ struct NvtxRange {
 namespace vmps {
 
 constexpr int kBlock = 256;
+// up to this many particles a FP64 solve forms p as it gathers (16 bytes an entry), above
+// it stores p (8 bytes, one more barrier of 2,400 to 3,400 cycles per iteration): us per
+// pass, formed against stored, 2D 1.9 k 3642 / 3926, 16 k 2369 / 2506, 29 k 1263 / 1297, 3D 24 k
+// 1816 / 1817, 54 k 897 / 887, 125 k 7030 / 6128, two-phase 86 k 5131 / 4987
+constexpr int kFormMax = 32768;
 
 // Cell grid of one support radius, NEIGHBOR's (functions.cu:2790-2802): x and
 // y cells of size re, z cells of size re + DELTA (3D).
@@ -241,8 +246,9 @@ struct mps_ctx {
     double* cg_part = nullptr;   // block partial sums
     size_t cg_part_cap = 0;      // doubles in cg_part
     double* cg_scal = nullptr;   // device scalars (rz, bb, rr, ...)
+    double2* cg_zp = nullptr;    // k_cg_loop: (z, p) of every row
     int* cg_flag = nullptr;      // [0] done, [1] iterations
-    unsigned int* cg_bar = nullptr;  // k_cg_loop's grid barrier: arrivals, monotonic per launch
+    unsigned int* cg_bar = nullptr;  // the one-launch solves' grid barrier: arrivals, monotonic per launch
     int* cg_flag_host = nullptr; // pinned
     double* red_host = nullptr;  // pinned scratch for scalars
     unsigned int* d_err = nullptr;

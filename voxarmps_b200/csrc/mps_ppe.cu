@@ -977,44 +977,447 @@ __global__ void k_ir_commit(double* scal, int* flag, double tol2, int use_cond,
 // ---------------------------------------------------------------------------
 // The whole solve in one cooperative launch, one block per SM, for systems whose
 // iterations cost more in launches, re-read partial sums and their gaps than in
-// bytes.  A block owns chunks of 32 rows, dealt out in turn (contiguous ranges
-// would leave the blocks of wall rows idle): their x, r,
-// direction, product and diagonal stay in its shared memory from the first
-// iteration to the last, and only the preconditioned residual z, which the
-// product gathers, and the block sums pass through memory.
+// bytes.  A block keeps the vectors of its rows in shared memory from the first
+// iteration to the last; only what other blocks gather passes through memory.
 //
-// CG in Chronopoulos and Gear's form (s-step methods, 1989): the product is
-// taken of z, s = A p follows by the recurrence s = w + beta s, and p.s from
-// z.w, so an iteration has two grid-wide synchronisations (the block sums of
-// z.w; z and the block sums of r.z and r.r) where the textbook form has three,
-// or four launches.  In exact arithmetic the iterates are the textbook form's.
+// FP64 (k_cg_loop): the launches' own operations in the launches' own order,
+// the block sums over the same virtual grid of 256-thread blocks, so the solution has the
+// launches' bits.  A scene may multiply a difference in the last bit by 1e6 within
+// a few steps (Herschel-Bulkley viscosity grows as 1 / sqrt(II) where the shear II
+// vanishes), so the form of the launch must not show in the result.
 //
-// Barriers: arrivals on one counter that grows by the grid size per barrier;
-// each wait is bounded (kBarSpins polls, about a second), past which the block
-// sets MPS_ERR_NOT_CONVERGED and leaves, so a lost block ends the solve instead
-// of hanging the GPU.
+// Mixed precision (k_ir_loop), whose inner iterations round to FP32 anyway: CG in
+// Chronopoulos and Gear's form (s-step methods, 1989): the product is taken of z,
+// s = A p follows by the recurrence s = w + beta s, and p.s from z.w.  In exact
+// arithmetic the iterates are the textbook form's; the refinements' FP64
+// residuals decide, as in the launches.
 //
-// G lanes per row: 8 in 2D (about 40 entries a row), 16 in 3D; four entries of a
-// lane in flight.  Two-phase scene, 86 k rows: 15 us per iteration (8 lanes; 16
-// lanes 1.5% more per step, 32 lanes 30%) against 29 us in four launches; 345 k rows
-// of 64 scenes in mixed precision 2797 us per step with 8 lanes, 3296 with 16.
+// Either has two grid-wide synchronisations per iteration.  Barriers: arrivals on one
+// counter that grows by the grid size per barrier; each wait is bounded (kBarPolls,
+// about a second and a half), past which the block sets MPS_ERR_NOT_CONVERGED and
+// leaves, so a lost block ends the solve instead of hanging the GPU.
 constexpr int kLoopThreads = 1024;
 
-constexpr long kBarSpins = 1L << 21;
 constexpr int kLoopMinRows = 64;    // rows per block at least (1.9 k rows: 32 rows 229 us per
                                     // step, 64 227, 128 234, 256 249)
 // scenes of up to this many particles solve in one block, without a grid-wide
 // synchronisation (a step from host arrays of 336 particles 239 -> 209 us; 663 particles
 // 171 us per step in one block or several, 1,093 235 against 182)
 constexpr int kLoopOneBlock = 512;
-// shared memory per row: six (k_ir_loop: three) doubles, (offset, length), five floats
-constexpr int kCgLoopRow = 6 * 8 + 8, kIrLoopRow = 3 * 8 + 8 + 5 * 4;
+// shared memory per row of the mixed solve: three doubles, (offset, length), five floats
+constexpr int kIrLoopRow = 3 * 8 + 8 + 5 * 4;
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p)
 {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
+}
+
+constexpr unsigned kBarPolls = 1u << 21;
+
+// one thread's wait until `target` blocks have arrived; past the limit the failure goes
+// to the error word and to the block's *fail
+__device__ __forceinline__ void wait_arrivals(unsigned* bar, unsigned target, unsigned* err,
+                                              int* fail)
+{
+    for (unsigned spins = 0; ld_acquire_u32(bar) < target;) {
+        if (++spins > kBarPolls) {
+            set_error(err, MPS_ERR_NOT_CONVERGED);
+            *fail = 1;
+            break;
+        }
+    }
+}
+
+struct Loop {
+    CG A;
+    int rows;         // k_ir_loop: rows per block
+    const double* b;  // right-hand side
+    const int* bcon;
+    double *x, *r, *z;
+    double* part;
+    double* scal;
+    int* flag;
+    unsigned *bar, *err;
+    double tol2;
+    int maxit;
+    int formed;       // r = b - A x0 is formed; x still holds the guess of every row
+    double pmin, pmax;
+    // k_cg_loop: the products' rows, A p, (z, p) of every row; slots per block of the
+    // vectors and of the product's rows
+    double* s;
+    double* p;
+    double2* zp;
+    int vslots, pslots;
+    // batched scenes (null for one): each row's scene, the scenes' slot ranges, caps,
+    // b.b and r.r, and whether each has converged
+    const int *scene, *first, *last;
+    const double* spmax;
+    double *sbb, *srr;
+    int* sok;
+    int nscenes;
+};
+
+// clamp of one pressure (functions.cu:2534-2547)
+__device__ __forceinline__ double clamp_p(double v, double pmin, double pmax)
+{
+    if (v < pmin) v = pmin;
+    if (v > pmax || v * 0.0 != 0.0) v = pmax;
+    return v;
+}
+
+// The virtual grid of a FP64 solve: A.nparts blocks of kRedThreads threads, the
+// launches' grid.  Virtual block b takes in sweep k the rows (b + k * A.nparts) *
+// width on: 256 rows of the vectors, 16 of the products.  Those past the last row
+// have none and add nothing to a sum.  They are dealt out to the blocks in turn
+// (runs of 4 to a block leave the blocks of wall rows idle: 125 k rows 6128 against 6367
+// us per pass).
+constexpr int kLoopVirtual = 32;  // virtual blocks per block at most
+struct Virtual {
+    int blocks;  // virtual blocks that have rows
+    int grid;    // blocks
+    int each;    // virtual blocks per block at most
+    int sweeps;  // sweeps of the grid
+    // block b's m-th virtual block, and how many it has
+    __host__ __device__ int at(int b, int m) const { return m * grid + b; }
+    __host__ __device__ int count(int b) const { return (blocks - b + grid - 1) / grid; }
+};
+__host__ __device__ inline Virtual virtual_grid(int n, int nparts, int width, int grid)
+{
+    Virtual v;
+    v.blocks = (n + width - 1) / width < nparts ? (n + width - 1) / width : nparts;
+    v.grid = grid;
+    v.each = (v.blocks + grid - 1) / grid;
+    v.sweeps = (int)((n + (long)nparts * width - 1) / ((long)nparts * width));
+    return v;
+}
+
+// Where a product's p comes from: stored, or z + beta p formed as it is gathered
+struct Stored {
+    const double* p;
+    typedef double Item;
+    __device__ __forceinline__ Item load(int j) const { return p[j]; }
+    __device__ __forceinline__ double value(Item v) const { return v; }
+};
+struct Formed {
+    const double2* zp;
+    double beta;
+    typedef double2 Item;
+    __device__ __forceinline__ Item load(int j) const { return zp[j]; }
+    __device__ __forceinline__ double value(Item v) const { return v.x + beta * v.y; }
+};
+
+// (A p)_i and p_i: the products and sums of spmv_row<16> in its order, by 16 lanes or by 8
+// that take the place of two each (entry j of a lane goes to the place j & 1, and
+// there to the first or the second sum in turn); four entries per lane in flight (one
+// block of 32 warps per SM leaves each warp 64 registers and needs the loads)
+template <int G, typename P>
+__device__ __forceinline__ double spmv_row_of(const CG& A, const Grp<G>& q, const P& p, int i,
+                                              int off, int L, double di, double& pi)
+{
+    static_assert(G == 16 || G == 8, "16 lanes, or two places of them each");
+    const int* __restrict__ c = A.mcol + off;
+    const double* __restrict__ a = A.mval + off;
+    const typename P::Item none{}, wi = p.load(i);
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    constexpr int S1 = 1, S2 = G == 16 ? 0 : 2, S3 = G == 16 ? 1 : 3;
+    for (int k = q.lane; k < L; k += 4 * G) {
+        const bool h1 = k + G < L, h2 = k + 2 * G < L, h3 = k + 3 * G < L;
+        const int c0 = c[k], c1 = h1 ? c[k + G] : 0, c2 = h2 ? c[k + 2 * G] : 0,
+                  c3 = h3 ? c[k + 3 * G] : 0;
+        const double a0 = a[k], a1 = h1 ? a[k + G] : 0.0, a2 = h2 ? a[k + 2 * G] : 0.0,
+                     a3 = h3 ? a[k + 3 * G] : 0.0;
+        const typename P::Item w0 = p.load(c0), w1 = h1 ? p.load(c1) : none,
+                               w2 = h2 ? p.load(c2) : none, w3 = h3 ? p.load(c3) : none;
+        s[0] += a0 * p.value(w0);
+        if (h1) s[S1] += a1 * p.value(w1);
+        if (h2) s[S2] += a2 * p.value(w2);
+        if (h3) s[S3] += a3 * p.value(w3);
+    }
+    pi = p.value(wi);
+    const double acc = q.sum(G == 16 ? s[0] + s[1] : (s[0] + s[2]) + (s[1] + s[3]));
+    return di * pi + acc;
+}
+
+// FP64: k_cg_start_rows, k_cg_spmv, k_cg_update, k_cg_direction and k_clamp in one
+// launch, with their bits.
+//
+// Products: any lane group takes any of the block's unknowns' rows (they are listed
+// once, so that every group has as many); p_i s_i goes to the row's slot, and the slots
+// are added in block_sum's order behind it.  Vectors: quarter h of the block (256
+// threads) runs the block's virtual blocks h, h + 4, ...
+//
+// STORE: the direction is stored by its row's owner, behind a barrier of its own.  Else
+// the owner publishes (z, p) and whoever gathers forms z + beta p, which saves the
+// textbook form its third synchronisation but gathers twice the bytes (kFormMax).
+//
+// G lanes per row: 16; in 2D (about 40 entries a row) 8 when p is stored or the grid is one
+// block (165 k rows 1801 us per pass against 1880; 1.9 k rows 4222 against 3926).
+// Bound by the exchanges in small scenes (1.9 k rows: 13,000 of 15,000 cycles per
+// iteration), by the matrix stream from L2 in large ones (two-phase scene, 86 k rows:
+// 24.6 us per iteration against 37.7 in four launches).
+template <int G, bool ONE, bool STORE>
+__global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(Loop L)
+{
+    constexpr int H = kLoopThreads / kRedThreads, W = kRedThreads / 32;
+    constexpr int GV = 2 * W;  // rows of a virtual block per sweep: 16 lanes each
+    extern __shared__ double sm[];
+    __shared__ double s_warp[3][kLoopVirtual][W], s_fin[3][W], s_tot[4];
+    __shared__ int s_fail, s_cnt[kLoopThreads / 32];
+    // what blocks exchange through memory: sums, products, (z, p).  One block
+    // by itself keeps them in shared memory
+    __shared__ double s_part[ONE ? 5 * kLoopVirtual : 1], s_prod[ONE ? kLoopOneBlock : 1];
+    __shared__ double2 s_zp[ONE ? kLoopOneBlock : 1];
+    const CG& A = L.A;
+    const int nv = A.nparts, pitch = ONE ? kLoopVirtual : nv;
+    double* const part = ONE ? s_part : L.part;
+    double* const prod = ONE ? s_prod : L.s;
+    double2* const zp = ONE ? s_zp : L.zp;
+    auto read = [](const double* a) { return ONE ? *a : __ldcg(a); };
+    const Virtual vec = virtual_grid(A.n, nv, kRedThreads, gridDim.x);
+    const Virtual pro = virtual_grid(A.n, nv, GV, gridDim.x);
+    const int t = threadIdx.x & (kRedThreads - 1), h = threadIdx.x / kRedThreads;
+    const int lane = threadIdx.x & 31, wv = t >> 5;
+    const Grp<G> q;
+    const int vm = vec.count(blockIdx.x), pm = pro.count(blockIdx.x);
+    double *sx = sm, *sr = sx + L.vslots, *sz = sr + L.vslots, *sp = sz + L.vslots,
+           *sd = sp + L.vslots, *pd = sd + L.vslots, *pps = pd + L.pslots;
+    int2* prow = reinterpret_cast<int2*>(pps + L.pslots);  // (offset, length) of an unknown's row
+    int2* pat = prow + L.pslots;                           // (row, slot in pps)
+    if (threadIdx.x == 0) s_fail = 0;
+    unsigned target = 0;
+    // the slot of (virtual block m, sweep k) of the vectors at this thread, and its row
+    auto slot = [&](int m, int k) { return (m * vec.sweeps + k) * kRedThreads + t; };
+    auto row = [&](int m, int k) { return (vec.at(blockIdx.x, m) + k * nv) * kRedThreads + t; };
+    // one value per thread of virtual block m, summed over each warp as block_sum does
+    auto put = [&](int j, int m, double v) {
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0) s_warp[j][m][wv] = v;
+    };
+    auto barrier = [&]() {
+        __syncthreads();
+        if (ONE) return true;
+        target += gridDim.x;
+        if (threadIdx.x == 0) {
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(L.bar) : "memory");
+            wait_arrivals(L.bar, target, L.err, &s_fail);
+        }
+        __syncthreads();
+        return s_fail == 0;
+    };
+    // the sums of `all` virtual blocks in the arrays first, first + 1, ..., added in
+    // reduce_parts' order; total j goes to done(j, total) in one thread
+    auto totals = [&](int count, int all, int first, auto done) {
+        if (h < count) {
+            const double* sums = part + (first + h) * pitch;
+            double v = 0.0;
+            for (int k = t; k < all; k += 8 * kRedThreads) {
+                double w[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    w[j] = k + j * kRedThreads < all ? read(sums + k + j * kRedThreads) : 0.0;
+#pragma unroll
+                for (int j = 0; j < 8; j++) v += w[j];
+            }
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) s_fin[h][wv] = v;
+        }
+        __syncthreads();
+        if (h < count && t == 0) {
+            double r = 0.0;
+            for (int k = 0; k < W; k++) r += s_fin[h][k];
+            done(h, r);
+        }
+        __syncthreads();
+    };
+    // the vectors' `count` values that put() left: this block's virtual blocks' sums, and
+    // the grid barrier behind them
+    auto share = [&](int count) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < count * vm; e += kLoopThreads) {
+            const int j = e / vm, m = e - j * vm;
+            double r = 0.0;
+            for (int k = 0; k < W; k++) r += s_warp[j][m][k];
+            part[j * pitch + vec.at(blockIdx.x, m)] = r;
+        }
+        return barrier();
+    };
+    // start: z = M^-1 r, p = z + 0 p
+    unsigned live = 0;  // bit u: this thread's u-th slot is an unknown
+    int u = 0;
+    for (int m = h; m < vm; m += H) {
+        double bb = 0, rz = 0, rr = 0;
+        for (int k = 0; k < vec.sweeps; k++, u++) {
+            const int i = row(m, k), at = slot(m, k);
+            if (i >= A.n) continue;
+            double xi = L.x[i], zi = 0.0;
+            if (A.bcon[i] == 0) {
+                const double bi = L.b[i], di = A.diag[i], ri = L.r[i];
+                zi = A.precond ? ri / di : ri;
+                bb += bi * bi;
+                rz += ri * zi;
+                rr += ri * ri;
+                live |= 1u << u;
+                sr[at] = ri;
+                sz[at] = zi;
+                sd[at] = di;
+            } else if (L.formed && L.bcon[i] != 0) {
+                xi = 0.0;
+            }
+            sx[at] = xi;
+            sp[at] = STORE ? zi : -0.0;
+            if (STORE) L.p[i] = zi;
+            else zp[i] = make_double2(zi, -0.0);  // z + 0 * -0 = z, whatever z's sign
+        }
+        __syncwarp();
+        put(0, m, bb);
+        put(1, m, rz);
+        put(2, m, rr);
+    }
+    // the product's rows: the unknowns among the block's, in their order, so that every
+    // lane group has as many
+    int rows = 0;
+    for (int e0 = 0; e0 < pm * pro.sweeps * GV; e0 += kLoopThreads) {
+        const int e = e0 + threadIdx.x;
+        int2 r = make_int2(0, -1);
+        int i = 0;
+        if (e < pm * pro.sweeps * GV) {
+            const int mk = e / GV, m = mk / pro.sweeps, k = mk - m * pro.sweeps;
+            i = (pro.at(blockIdx.x, m) + k * nv) * GV + (e - mk * GV);
+            if (i < A.n) r = A.mrow[i];
+            pps[e] = 0.0;
+        }
+        const unsigned who = __ballot_sync(0xffffffffu, r.y >= 0);
+        if (lane == 0) s_cnt[threadIdx.x >> 5] = __popc(who);
+        __syncthreads();
+        int before = rows;
+        for (int w = 0; w < kLoopThreads / 32; w++) {
+            if (w < (int)(threadIdx.x >> 5)) before += s_cnt[w];
+            rows += s_cnt[w];
+        }
+        if (r.y >= 0) {
+            const int c = before + __popc(who & ((1u << lane) - 1u));
+            prow[c] = r;
+            pat[c] = make_int2(i, e);
+            pd[c] = A.diag[i];
+        }
+        __syncthreads();
+    }
+    double bb, rz, rr, beta = 0.0;
+    bool ok;
+    if (L.formed) {
+        ok = share(3);
+        totals(3, vec.blocks, 0, [&](int j, double v) { s_tot[j] = v; });
+        bb = s_tot[0];
+        rz = s_tot[1];
+        rr = s_tot[2];
+        if (ok && blockIdx.x == 0 && threadIdx.x == 0) {
+            L.scal[S_BB] = bb;
+            L.scal[S_RR] = L.scal[S_RR0] = rr;
+            L.scal[S_ZERO] = bb == 0.0 ? 1.0 : 0.0;
+        }
+    } else {  // k_cg_start has the sums
+        bb = L.scal[S_BB];
+        rz = L.scal[S_RZ];
+        rr = L.scal[S_RR];
+        ok = barrier();
+    }
+    bool done = bb == 0.0 || rr <= L.tol2 * bb;
+    int it = 0;
+    while (ok && !done) {
+        // s = A p, p.s
+        for (int c = threadIdx.x / G; c < rows; c += kLoopThreads / G) {
+            const int2 r = prow[c], at = pat[c];
+            double pi;
+            const double si =
+                STORE ? spmv_row_of(A, q, Stored{L.p}, at.x, r.x, r.y, pd[c], pi)
+                      : spmv_row_of(A, q, Formed{zp, beta}, at.x, r.x, r.y, pd[c], pi);
+            if (q.lane == 0) {
+                prod[at.x] = si;
+                pps[at.y] = pi * si;
+            }
+        }
+        __syncthreads();
+        // a virtual block's p.s in block_sum's order: each row group's over the sweeps, the
+        // two of a warp, the warps
+        for (int e0 = 0; e0 < pm * GV; e0 += kLoopThreads) {
+            const int e = e0 + threadIdx.x, m = e / GV, g = e - m * GV;
+            double v = 0.0;
+            if (m < pm)
+                for (int k = 0; k < pro.sweeps; k++) v += pps[(m * pro.sweeps + k) * GV + g];
+            v += __shfl_down_sync(0xffffffffu, v, 1);
+            double r = 0.0;
+            for (int w = 0; w < W; w++) r += __shfl_sync(0xffffffffu, v, (lane & GV) + 2 * w);
+            if (m < pm && g == 0) part[4 * pitch + pro.at(blockIdx.x, m)] = r;
+        }
+        if (!(ok = barrier())) break;
+        // (a thread's first product travels beside the sums)
+        const double s0 = live & 1u ? read(prod + row(h, 0)) : 0.0;
+        totals(1, pro.blocks, 4, [&](int, double v) { s_tot[0] = rz / v; });
+        // x += alpha p, r -= alpha s, z = M^-1 r, r.z, r.r
+        const double alpha = s_tot[0];
+        u = 0;
+        for (int m = h; m < vm; m += H) {
+            double rz1 = 0, rr1 = 0;
+            for (int k = 0; k < vec.sweeps; k++, u++) {
+                if (!(live >> u & 1u)) continue;
+                const int i = row(m, k), at = slot(m, k);
+                const double si = u == 0 ? s0 : read(prod + i);
+                const double pk = STORE ? sp[at] : sz[at] + beta * sp[at];
+                const double xi = sx[at] + alpha * pk;
+                const double ri = sr[at] - alpha * si;
+                const double zi = A.precond ? ri / sd[at] : ri;
+                sx[at] = xi;
+                sr[at] = ri;
+                sz[at] = zi;
+                if (!STORE) {
+                    sp[at] = pk;
+                    zp[i] = make_double2(zi, pk);
+                }
+                rz1 += ri * zi;
+                rr1 += ri * ri;
+            }
+            __syncwarp();
+            put(0, m, rz1);
+            put(1, m, rr1);
+        }
+        if (!(ok = share(2))) break;
+        // beta by one thread: a division in each of 1024 threads is 600 cycles of FP64 issue
+        totals(2, vec.blocks, 0, [&](int j, double v) {
+            s_tot[1 + j] = v;
+            if (j == 0) s_tot[3] = v / rz;
+        });
+        rz = s_tot[1];
+        rr = s_tot[2];
+        beta = s_tot[3];
+        it++;
+        done = rr <= L.tol2 * bb || it >= L.maxit || !(rr == rr);
+        if (STORE && !done) {
+            u = 0;
+            for (int m = h; m < vm; m += H)
+                for (int k = 0; k < vec.sweeps; k++, u++)
+                    if (live >> u & 1u) {
+                        const int at = slot(m, k);
+                        const double pk = sz[at] + beta * sp[at];
+                        sp[at] = pk;
+                        L.p[row(m, k)] = pk;
+                    }
+            ok = barrier();
+        }
+    }
+    if (ok && blockIdx.x == 0 && threadIdx.x == 0) {
+        L.scal[S_RR] = rr;
+        L.flag[0] = 1;
+        L.flag[1] = it;
+    }
+    // the solution back, clamped; a zero right-hand side gives p = 0
+    for (int m = h; m < vm; m += H)
+        for (int k = 0; k < vec.sweeps; k++) {
+            const int i = row(m, k);
+            if (i < A.n)
+                L.x[i] = clamp_p(ok && bb == 0.0 ? 0.0 : sx[slot(m, k)], L.pmin, L.pmax);
+        }
 }
 
 // ONE: the grid is one block, whose sums are the totals
@@ -1089,55 +1492,13 @@ struct Sync {
         __syncthreads();
         return *fail == 0;
     }
-    __device__ __forceinline__ void wait()
-    {
-        long spins = 0;
-        while (ld_acquire_u32(bar) < target) {
-            if (++spins > kBarSpins) {
-                set_error(err, MPS_ERR_NOT_CONVERGED);
-                *fail = 1;
-                break;
-            }
-        }
-        __threadfence();
-    }
-};
-
-struct Loop {
-    CG A;
-    int rows;         // rows per block
-    const double* b;  // right-hand side
-    const int* bcon;
-    double *x, *r, *z;
-    double* part;
-    double* scal;
-    int* flag;
-    unsigned *bar, *err;
-    double tol2;
-    int maxit;
-    int formed;       // r = b - A x0 is formed; x still holds the guess of every row
-    double pmin, pmax;
-    // batched scenes (null for one): each row's scene, the scenes' slot ranges, caps,
-    // b.b and r.r, and whether each has converged
-    const int *scene, *first, *last;
-    const double* spmax;
-    double *sbb, *srr;
-    int* sok;
-    int nscenes;
+    __device__ __forceinline__ void wait() { wait_arrivals(bar, target, err, fail); }
 };
 
 // the block's k-th row: chunks of 32 rows dealt out to the blocks in turn
 __device__ __forceinline__ int loop_row(int k)
 {
     return ((k >> 5) * (int)gridDim.x + (int)blockIdx.x) * 32 + (k & 31);
-}
-
-// clamp of one pressure (functions.cu:2534-2547)
-__device__ __forceinline__ double clamp_p(double v, double pmin, double pmax)
-{
-    if (v < pmin) v = pmin;
-    if (v > pmax || v * 0.0 != 0.0) v = pmax;
-    return v;
 }
 
 // the solution back, clamped; a zero right-hand side gives p = 0
@@ -1156,119 +1517,14 @@ __device__ __forceinline__ void loop_finish(const Loop& L, const double* sx, boo
     }
 }
 
-template <int G, bool ONE>
-__global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(Loop L)
-{
-    extern __shared__ double sm[];
-    __shared__ double s_warp[3][32], s_tot[3];
-    // alpha, beta, beta r.z / alpha by one thread: three divisions in each of 1024
-    // threads are 1,700 cycles of FP64 issue (86 k rows 1118 -> 1096 us per step;
-    // k_ir_loop, in whose registers they lie better, loses 3% by it)
-    __shared__ double s_coef[3];
-    __shared__ int s_fail;
-    const CG& A = L.A;
-    const int R = L.rows, nr = R;
-    // the block's k-th row
-    auto row = [](int k) { return loop_row(k); };
-    double *sx = sm, *sr = sx + R, *sp = sr + R, *ss = sp + R, *sw = ss + R, *sd = sw + R;
-    int2* srow = reinterpret_cast<int2*>(sd + R);
-    if (threadIdx.x == 0) {
-        s_fail = 0;
-        s_coef[1] = s_coef[2] = 0.0;
-    }
-    Sync<ONE> sync{L.bar, L.err, L.part, 0u, s_warp, s_tot, &s_fail};
-    // start: z = M^-1 r, p = s = 0
-    double v[3] = {0, 0, 0};
-    for (int k = threadIdx.x; k < nr; k += kLoopThreads) {
-        const int i = row(k);
-        srow[k] = make_int2(0, -1);
-        if (i >= A.n) continue;
-        const int2 m = A.mrow[i];
-        double xi = L.x[i], ri = 0, zi = 0;
-        if (m.y >= 0) {
-            const double bi = L.b[i], di = A.diag[i];
-            ri = L.r[i];
-            zi = A.precond ? ri / di : ri;
-            v[0] += bi * bi;
-            v[1] += ri * zi;
-            v[2] += ri * ri;
-            sd[k] = di;
-        } else if (L.formed && L.bcon[i] != 0) {
-            xi = 0.0;
-        }
-        srow[k] = m;
-        sx[k] = xi;
-        sr[k] = ri;
-        sp[k] = ss[k] = 0.0;
-        L.z[i] = zi;
-    }
-    if (!sync.sums<3>(v, 0)) return;
-    const double bb = v[0];
-    double rz = v[1], rr = v[2], rz_old = rz, alpha = 1.0;
-    bool done = bb == 0.0 || rr <= L.tol2 * bb;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        L.scal[S_BB] = bb;
-        L.scal[S_RR0] = rr;
-        L.scal[S_ZERO] = bb == 0.0 ? 1.0 : 0.0;
-    }
-    const Grp<G> q;
-    const int grp = threadIdx.x / G;
-    int it = 0;
-    while (!done) {
-        if (it > 0 && threadIdx.x == kLoopThreads - 1) {  // beside the product
-            const double beta = rz / rz_old;
-            s_coef[1] = beta;
-            s_coef[2] = beta * rz / alpha;
-        }
-        // w = A z and z.w
-        double zw[1] = {0};
-        for (int k = grp; k < nr; k += kLoopThreads / G) {
-            const int2 m = srow[k];
-            if (m.y < 0) continue;
-            const double wi = spmv_row4(A, q, L.z, row(k), m.x, m.y, sd[k]);
-            if (q.lane == 0) {
-                sw[k] = wi;
-                zw[0] += L.z[row(k)] * wi;
-            }
-        }
-        if (!sync.sums<1>(zw, 3)) return;
-        if (threadIdx.x == 0) s_coef[0] = rz / (zw[0] - s_coef[2]);
-        __syncthreads();
-        alpha = s_coef[0];
-        const double beta = s_coef[1];
-        v[0] = v[1] = 0.0;
-        for (int k = threadIdx.x; k < nr; k += kLoopThreads) {
-            if (srow[k].y < 0) continue;
-            const double r0 = sr[k], z0 = A.precond ? r0 / sd[k] : r0;
-            const double pk = z0 + beta * sp[k], sk = sw[k] + beta * ss[k];
-            const double r1 = r0 - alpha * sk, z1 = A.precond ? r1 / sd[k] : r1;
-            sp[k] = pk;
-            ss[k] = sk;
-            sx[k] += alpha * pk;
-            sr[k] = r1;
-            L.z[row(k)] = z1;
-            v[0] += r1 * z1;
-            v[1] += r1 * r1;
-        }
-        if (!sync.sums<2>(v, 4)) return;
-        rz_old = rz;
-        rz = v[0];
-        rr = v[1];
-        it++;
-        done = rr <= L.tol2 * bb || it >= L.maxit || !(rr == rr);
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        L.scal[S_RR] = rr;
-        L.flag[0] = 1;
-        L.flag[1] = it;
-    }
-    loop_finish(L, sx, bb == 0.0);
-}
-
-// The mixed-precision solve (the sweeps described above) in the same form: FP32
+// The mixed-precision solve (the sweeps described above) in one launch: FP32
 // inner CG with the FP32 vectors, x and r in shared memory; z and, for a
-// refinement's product, d pass through memory.  Batched scenes: each scene's
-// r.r is summed over its slot range after a refinement, a block per scene.
+// refinement's product, d pass through memory.  A block owns chunks of 32 rows,
+// dealt out in turn (contiguous ranges would leave the blocks of wall rows
+// idle).  Batched scenes: each scene's r.r is summed over its slot range after a
+// refinement, a block per scene.
+// G lanes per row: 8 in 2D (about 40 entries a row), 16 in 3D; four entries of a
+// lane in flight (345 k rows of 64 scenes 2797 us per step with 8 lanes, 3296 with 16).
 template <int G, bool ONE>
 __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
 {
@@ -1315,7 +1571,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
         I.z[i] = z32;
         I.d[i] = 0.f;
     }
-    if (!sync.sums<4>(v, 0)) return;
+    if (!sync.template sums<4>(v, 0)) return;
     const double bb = v[0];
     double rr = v[1], rz = v[2], rin0 = v[3], rz_old = rz, alpha = 1.0;
     double eta2 = sweep_target(L.tol2, bb, rr);
@@ -1340,7 +1596,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
                 zw[0] += (double)I.z[row(k)] * (double)wi;
             }
         }
-        if (!sync.sums<1>(zw, 4)) return;
+        if (!sync.template sums<1>(zw, 4)) return;
         const double beta = first ? 0.0 : rz / rz_old;
         alpha = first ? rz / zw[0] : rz / (zw[0] - beta * rz / alpha);
         first = false;
@@ -1359,7 +1615,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
             v[0] += (double)r1 * (double)z1;
             v[1] += (double)r1 * (double)r1;
         }
-        if (!sync.sums<2>(v, 5)) return;
+        if (!sync.template sums<2>(v, 5)) return;
         rz_old = rz;
         rz = v[0];
         const double rin = v[1];
@@ -1393,7 +1649,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
             v[1] += (double)r32 * (double)z32;
             v[2] += (double)r32 * (double)r32;
         }
-        if (!sync.sums<3>(v, 7)) return;
+        if (!sync.template sums<3>(v, 7)) return;
         rr = v[0];
         rz = v[1];
         rin0 = v[2];
@@ -1413,9 +1669,9 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
                 }
             }
             if (!sync.all()) return;
-            bool ok = true;
-            for (int k = threadIdx.x; k < L.nscenes; k += kLoopThreads) ok = ok && __ldcg(L.sok + k) != 0;
-            conv = __syncthreads_and(ok) != 0;
+            bool all = true;
+            for (int k = threadIdx.x; k < L.nscenes; k += kLoopThreads) all = all && __ldcg(L.sok + k) != 0;
+            conv = __syncthreads_and(all) != 0;
         }
         sweeps++;
         done = conv || it >= L.maxit || sweeps >= kMaxSweeps || !(rr == rr);
@@ -1544,40 +1800,84 @@ static int ppe_assemble(mps_ctx* c, int* warm_out, double* r0 = nullptr, bool* f
     return MPS_OK;
 }
 
-// grid of the CG kernels: blocks per SM from the autotuner, else as many as
-// fit (at most 8); cg_part holds [0,3*nblk) start/update partials and
-// [4*nblk,5*nblk) p.s
 // Scenes of at most this many particles solve in one cooperative launch (FP64
-// batches, whose scenes are tested every iteration, keep the launches).  Launches
-// against one launch, us per step: FP64 2D 1.9 k 282 / 229, two-phase 86 k 1870 /
-// 1174, 2D 165 k 1089 / 918; 3D 54 k 990 / 814, 125 k 1677 / 1610, 245 k 3095 /
-// 2947, 476 k 5187 / 5338 (from there the product is bound by HBM, which the
-// launches' 64 warps per SM load faster); mixed precision 2D 165 k 1390 / 1075, 3D
-// 125 k 2224 / 1825, 476 k 6355 / 5755.  Beyond, shared memory ends (52 or 56 bytes
-// per row).
-constexpr int kLoopMax = 300000, kIrLoopMax = 524288;
+// batches, whose scenes are tested every iteration, keep the launches).
+// Launches against one launch, us per step: FP64 2D 1.9 k 282 / 176, 16 k 367 / 229, 164 k
+// 1028 / 889; two-phase 12 k 1081 / 558, 86 k 1752 / 1183, 169 k 2401 / 1856; 3D 24 k 601 / 450,
+// 54 k 1277 / 874, 125 k 1551 / 1532, 233 k 3255 / 3197 (from 262,144 rows on the
+// launches' products take a whole warp per row, another order of sums, and gain as much
+// from it: 274 k 3707); mixed precision 2D 165 k 1390 / 1075, 3D 125 k 2224 / 1825, 476 k
+// 6355 / 5755, and beyond 524,288 shared memory ends (52 bytes per row).
+constexpr int kLoopMax = kNarrowMaxRows, kIrLoopMax = 524288;
 constexpr int kLoopMaxBytes = 200 * 1024;
-
-// blocks and rows per block of a one-launch solve
-static void loop_grid(const mps_ctx* c, int sms, int* nblk, int* rows)
+// the virtual grid of a FP64 solve of up to kSmallRows rows is 4 blocks per SM, and no
+// more than the rows' groups fill (it sets the order of the sums, so it stays as it is)
+constexpr int kSmallRows = 16384, kSmallBps = 4;
+// blocks of the CG kernels' grid: blocks per SM from the autotuner, else as many as fit
+// (at most 8), fewer for small FP64 systems; cg_part holds [0,3*nblk) start/update
+// partials and [4*nblk,5*nblk) p.s.  whole: a whole warp per row (the slabs)
+static int cg_grid(mps_ctx* c, int* out, bool whole = false)
 {
-    *nblk = c->n <= kLoopOneBlock ? 1 : std::min(sms, (c->n + kLoopMinRows - 1) / kLoopMinRows);
+    int nblk = 0, occ = 0;
+    const bool narrow = !whole && c->n <= kNarrowMaxRows;
+    VMPS_CUDA(c, cudaDeviceGetAttribute(&nblk, cudaDevAttrMultiProcessorCount, c->device));
+    VMPS_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                     &occ, narrow ? k_cg_spmv<16> : k_cg_spmv<kRowG>, kRedThreads, 0));
+    const bool small = !whole && c->cfg.precision == 0 && c->nscenes == 1 && c->n <= kSmallRows;
+    const int sms = nblk, bps = c->tune_cg_bps > 0 ? c->tune_cg_bps : 8;
+    nblk *= std::max(1, std::min(small ? std::min(occ, kSmallBps) : occ, bps));
+    if (small)
+        nblk = std::min(nblk, std::max(sms, (c->n + kRedThreads / 16 - 1) / (kRedThreads / 16)));
+    if ((size_t)5 * nblk > c->cg_part_cap) {
+        c->msg = "CG partial buffer too small for the launch grid";
+        return MPS_ERR_ARG;
+    }
+    *out = nblk;
+    return MPS_OK;
+}
+
+// blocks, slots and shared bytes of a one-launch solve
+struct LoopShape {
+    int blocks, rows, vslots, pslots, bytes;
+    bool fits;
+};
+static LoopShape loop_shape(const mps_ctx* c, int sms, int nparts)
+{
+    LoopShape s{};
+    s.blocks = c->n <= kLoopOneBlock ? 1 : std::min(sms, (c->n + kLoopMinRows - 1) / kLoopMinRows);
     const int chunks = (c->n + 31) / 32;
-    *rows = (chunks + *nblk - 1) / *nblk * 32;
+    s.rows = (chunks + s.blocks - 1) / s.blocks * 32;
+    if (c->cfg.precision >= 1) {
+        s.bytes = s.rows * kIrLoopRow;
+        s.fits = s.bytes <= kLoopMaxBytes;
+        return s;
+    }
+    const Virtual vec = virtual_grid(c->n, nparts, kRedThreads, s.blocks);
+    const Virtual pro = virtual_grid(c->n, nparts, kRedThreads / 16, s.blocks);
+    s.vslots = vec.each * vec.sweeps * kRedThreads;
+    s.pslots = pro.each * pro.sweeps * (kRedThreads / 16);
+    s.bytes = (s.vslots * 5 + s.pslots * 4) * (int)sizeof(double);
+    // (a thread's slots are the bits of a word)
+    s.fits = s.bytes <= kLoopMaxBytes && std::max(vec.each, pro.each) <= kLoopVirtual &&
+             (vec.each + 3) / 4 * vec.sweeps <= 32;
+    return s;
 }
 
 static bool use_cg_loop(mps_ctx* c)
 {
     const bool mixed = c->cfg.precision >= 1;
-    if ((!mixed && c->nscenes > 1) || c->n > (mixed ? kIrLoopMax : kLoopMax)) return false;
-    int coop = 0, sms = 0, nblk, rows;
+    if ((!mixed && c->nscenes > 1) || c->n > (mixed ? kIrLoopMax : kLoopMax))
+        return false;
+    // mixed precision: the launch's sums and recurrence are its own, and a
+    // non-Newtonian scene magnifies any difference of rounding
+    if (mixed && c->cfg.fluid2_type != 0) return false;
+    int coop = 0, sms = 0, nparts = 0;
     if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    loop_grid(c, sms, &nblk, &rows);
-    return coop != 0 && rows * (mixed ? kIrLoopRow : kCgLoopRow) <= kLoopMaxBytes;
+    return coop != 0 && cg_grid(c, &nparts) == MPS_OK && loop_shape(c, sms, nparts).fits;
 }
 
 static int launch_loop(mps_ctx* c, const CG& A, const IR& I, double tol2, bool formed)
@@ -1586,49 +1886,59 @@ static int launch_loop(mps_ctx* c, const CG& A, const IR& I, double tol2, bool f
     int sms = 0;
     VMPS_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
     const bool mixed = f.precision >= 1, batched = c->nscenes > 1, three = f.dim == 3;
-    int nblk = 0, rows = 0;
-    loop_grid(c, sms, &nblk, &rows);
-    const int bytes = rows * (mixed ? kIrLoopRow : kCgLoopRow);
-    const bool one = nblk == 1;
+    const LoopShape s = loop_shape(c, sms, A.nparts);
+    const bool one = s.blocks == 1, form = c->n <= kFormMax;
     const void* fn =
         mixed ? (three ? (one ? (const void*)k_ir_loop<16, true> : (const void*)k_ir_loop<16, false>)
                        : (one ? (const void*)k_ir_loop<8, true> : (const void*)k_ir_loop<8, false>))
-              : (three ? (one ? (const void*)k_cg_loop<16, true> : (const void*)k_cg_loop<16, false>)
-                       : (one ? (const void*)k_cg_loop<8, true> : (const void*)k_cg_loop<8, false>));
+        : one  ? (three ? (const void*)k_cg_loop<16, true, false> : (const void*)k_cg_loop<8, true, false>)
+        : form ? (const void*)k_cg_loop<16, false, false>
+               : (three ? (const void*)k_cg_loop<16, false, true> : (const void*)k_cg_loop<8, false, true>);
     // (always the same bound: the attribute is the function's, for every context)
     VMPS_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       kLoopMaxBytes));
-    Loop L{A, rows, c->source, c->bcon, c->pnew, c->cg_r, c->cg_z, c->cg_part, c->cg_scal,
-           c->cg_flag, c->cg_bar, c->d_err, tol2, f.cg_max, formed ? 1 : 0, f.pmin, f.pmax,
-           batched ? c->scene : nullptr, c->sfirst, c->slast, c->spmax, c->sbb, c->srr, c->sok,
-           c->nscenes};
+    Loop L{};
+    L.A = A;
+    L.rows = s.rows;
+    L.b = c->source;
+    L.bcon = c->bcon;
+    L.x = c->pnew;
+    L.r = c->cg_r;
+    L.z = c->cg_z;
+    L.part = c->cg_part;
+    L.scal = c->cg_scal;
+    L.flag = c->cg_flag;
+    L.bar = c->cg_bar;
+    L.err = c->d_err;
+    L.tol2 = tol2;
+    L.maxit = f.cg_max;
+    L.formed = formed ? 1 : 0;
+    L.pmin = f.pmin;
+    L.pmax = f.pmax;
+    L.s = c->cg_s;
+    L.p = c->cg_p;
+    L.zp = c->cg_zp;
+    L.vslots = s.vslots;
+    L.pslots = s.pslots;
+    L.scene = batched ? c->scene : nullptr;
+    L.first = c->sfirst;
+    L.last = c->slast;
+    L.spmax = c->spmax;
+    L.sbb = c->sbb;
+    L.srr = c->srr;
+    L.sok = c->sok;
+    L.nscenes = c->nscenes;
     if (!one) VMPS_CUDA(c, cudaMemsetAsync(c->cg_bar, 0, sizeof(unsigned), c->stream));
     IR i = I;
     void* cg_args[] = {&L};
     void* ir_args[] = {&L, &i};
     if (one)
         VMPS_CUDA(c, cudaLaunchKernel(fn, dim3(1), dim3(kLoopThreads), mixed ? ir_args : cg_args,
-                                      bytes, c->stream));
+                                      s.bytes, c->stream));
     else
-        VMPS_CUDA(c, cudaLaunchCooperativeKernel(fn, dim3(nblk), dim3(kLoopThreads),
-                                                 mixed ? ir_args : cg_args, bytes, c->stream));
+        VMPS_CUDA(c, cudaLaunchCooperativeKernel(fn, dim3(s.blocks), dim3(kLoopThreads),
+                                                 mixed ? ir_args : cg_args, s.bytes, c->stream));
     vmps_count_launch(1);
-    return MPS_OK;
-}
-
-static int cg_grid(mps_ctx* c, int* out, int g = kRowG)
-{
-    int nblk = 0, occ = 0;
-    VMPS_CUDA(c, cudaDeviceGetAttribute(&nblk, cudaDevAttrMultiProcessorCount, c->device));
-    VMPS_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                     &occ, g == 16 ? k_cg_spmv<16> : k_cg_spmv<kRowG>, kRedThreads, 0));
-    const int bps = c->tune_cg_bps > 0 ? c->tune_cg_bps : 8;
-    nblk *= std::max(1, std::min(occ, bps));
-    if ((size_t)5 * nblk > c->cg_part_cap) {
-        c->msg = "CG partial buffer too small for the launch grid";
-        return MPS_ERR_ARG;
-    }
-    *out = nblk;
     return MPS_OK;
 }
 
@@ -1640,12 +1950,14 @@ int vmps_ppe(mps_ctx* c, bool report)
     const bool mixed = f.precision >= 1;
     int warm = 0, nblk = 0;
     bool fused = false;
-    const bool loop = use_cg_loop(c);  // the whole solve in one cooperative launch
+    // the whole solve in one cooperative launch; a profiled FP64 solve, whose
+    // products are timed, takes the launches, with the same bits
+    const bool loop = use_cg_loop(c) && (mixed || !c->profile);
     const bool narrow = n <= kNarrowMaxRows;  // 16 lanes per row in the FP64 products
     {
         int r = ppe_assemble(c, &warm, c->cg_r, &fused);
         if (r != MPS_OK) return r;
-        r = cg_grid(c, &nblk, narrow ? 16 : kRowG);
+        r = cg_grid(c, &nblk);
         if (r != MPS_OK) return r;
     }
     // zero initial guess (the assembly zeroed pnew): r = b exactly, so the
@@ -1977,7 +2289,7 @@ int mps_dcg_start(mps_ctx* c, double* local3)
     DCG_NEED(c);
     if (!local3) return MPS_ERR_ARG;
     int nblk = 0;
-    int r = cg_grid(c, &nblk);
+    int r = cg_grid(c, &nblk, true);
     if (r != MPS_OK) return r;
     const CG G = dcg_args(c, nblk);
     VMPS_CUDA(c, cudaMemsetAsync(c->cg_flag, 0, 4 * sizeof(int), c->stream));
@@ -1992,7 +2304,7 @@ int mps_dcg_spmv(mps_ctx* c, double* local_ps)
     DCG_NEED(c);
     if (!local_ps) return MPS_ERR_ARG;
     int nblk = 0;
-    int r = cg_grid(c, &nblk);
+    int r = cg_grid(c, &nblk, true);
     if (r != MPS_OK) return r;
     const CG G = dcg_args(c, nblk);
     k_cg_spmv<kRowG><<<nblk, kRedThreads, 0, c->stream>>>(G, c->cg_p, c->cg_s, c->cg_part + 4 * nblk,
@@ -2006,7 +2318,7 @@ int mps_dcg_update(mps_ctx* c, double alpha, double* local2)
     DCG_NEED(c);
     if (!local2) return MPS_ERR_ARG;
     int nblk = 0;
-    int r = cg_grid(c, &nblk);
+    int r = cg_grid(c, &nblk, true);
     if (r != MPS_OK) return r;
     const CG G = dcg_args(c, nblk);
     k_dcg_update<<<nblk, kRedThreads, 0, c->stream>>>(G, alpha, c->pnew, c->cg_r, c->cg_z,
@@ -2019,7 +2331,7 @@ int mps_dcg_direction(mps_ctx* c, double beta)
 {
     DCG_NEED(c);
     int nblk = 0;
-    int r = cg_grid(c, &nblk);
+    int r = cg_grid(c, &nblk, true);
     if (r != MPS_OK) return r;
     k_dcg_direction<<<nblk, kRedThreads, 0, c->stream>>>(dcg_args(c, nblk), beta, c->cg_z, c->cg_p);
     vmps_count_launch(1);
