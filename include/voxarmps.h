@@ -212,6 +212,12 @@ int mps_set_profile(mps_ctx* ctx, int on);
  * one graph launch and one host synchronisation per step.  Results are
  * identical to eager mode.  Off while profiling (mps_set_profile). */
 int mps_set_graph(mps_ctx* ctx, int on);
+/* Bound of a wait of the one-launch pressure solves' grid, in polls of its
+ * counter (0, the default: 2^21, about a second and a half).  A solve whose
+ * wait runs out is abandoned: the pressures are clamped and finite,
+ * cg_relres is NaN, cg_iters 0, MPS_ERR_NOT_CONVERGED is set, and
+ * mps_pressure returns it. */
+int mps_set_wait_limit(mps_ctx* ctx, unsigned int polls);
 
 /* ---- launch-shape autotuning (no reference counterpart) ------------------ *
  * small_lanes: lanes per row of the PND-radius list in the list build and

@@ -1,0 +1,93 @@
+"""A one-launch solve whose grid wait runs out (here by a limit of one poll, which the
+first exchange of 148 blocks exceeds) is reported as not converged, with the
+figures of no earlier solve, and leaves clamped pressures; the next solve, with
+the usual limit, converges."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import voxarmps_b200 as vm
+from voxarmps_b200 import cases, config
+from gpu_util import gpu_cfg
+
+pytestmark = pytest.mark.gpu
+
+NOT_CONVERGED = 64
+PMIN, PMAX = 0.0, 400.0
+
+
+def _dam(**kw):
+    l0 = 0.01
+    case = cases.dam_break(2, l0, (90, 110), (150, 120))
+    cfg = config.reference_defaults(l0, 2)
+    cfg.update(re_s=2.1 * l0, re_l=4.0 * l0, dt=1e-4, gy=-9.81)
+    return gpu_cfg(config.with_box(cfg, case), pmin=PMIN, pmax=PMAX, **kw), case, None
+
+
+def _batch(**kw):
+    l0 = 0.01
+    scenes = [cases.dam_break(2, l0, (w, h), (120, 70)) for w, h in ((60, 55), (25, 50), (90, 60))]
+    base = config.reference_defaults(l0, 2)
+    base.update(re_s=2.1 * l0, re_l=4.0 * l0, dt=1e-4, gy=-9.81)
+    cfg, case, sid, boxes, _ = config.batched(gpu_cfg(base, pmin=PMIN, pmax=PMAX, **kw), scenes)
+    return cfg, case, (sid, boxes, [PMAX] * len(scenes))
+
+
+def _solver(cfg, case, scenes):
+    s = vm.Solver(cfg, case)
+    if scenes is not None:
+        s.set_scenes(*scenes)
+    assert s.init() == 0
+    return s
+
+
+def _check(s):
+    assert np.isnan(s.scalar("cg_relres")) and s.scalar("cg_iters") == 0
+    p = s.get("pnew")
+    assert np.isfinite(p).all() and p.min() >= PMIN and p.max() <= PMAX
+    assert not p[s.get("bcon") != 0].any()
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("make, opts", [
+    (_dam, dict()), (_dam, dict(warm_start=0)), (_dam, dict(precision=1)),
+    (_batch, dict(precision=1))], ids=str)
+def test_step(make, opts, graph):
+    s = _solver(*make(**opts))
+    s.set_graph(graph)
+    for _ in range(2):  # both buffer sets
+        assert s.step() == 0
+    assert s.scalar("one_launch_solve") == 1 and s.scalar("cg_iters") >= 1
+    s.set_wait_limit(1)
+    for _ in range(2):
+        assert s.step() == NOT_CONVERGED
+        _check(s)
+    s.set_wait_limit()
+    for _ in range(2):
+        assert s.step() == 0
+        assert s.scalar("cg_iters") >= 1 and s.scalar("cg_relres") <= s.cfg["cg_tol"]
+    s.close()
+
+
+@pytest.mark.parametrize("opts", [dict(), dict(precision=1)], ids=str)
+def test_pressure_stage(opts):
+    s = _solver(*_dam(**opts))
+    assert s.step() == 0
+
+    def solve():
+        it, rr = C.c_int(-1), C.c_double(-1.0)
+        r = s.lib.mps_pressure(s.h, C.byref(it), C.byref(rr))
+        return r, it.value, rr.value
+
+    for name in ("neighbors", "vfraction", "viscosity", "predict", "pnd_star", "bcon"):
+        getattr(s, name)()
+    s.set_wait_limit(1)
+    r, it, rr = solve()
+    assert r == NOT_CONVERGED and it == 0 and np.isnan(rr)
+    _check(s)
+    s.set_wait_limit()
+    r, it, rr = solve()
+    assert r == 0 and it >= 1 and rr <= s.cfg["cg_tol"]
+    assert s.error() & NOT_CONVERGED  # the abandoned solve's
+    s.close()

@@ -45,7 +45,7 @@ EXPORTS = [
     "mps_download_lists", "mps_get_scalar", "mps_get_error", "mps_last_message",
     "mps_write_vtu", "mps_stream", "mps_set_state", "mps_get_state", "mps_step_io",
     "mps_set_field",
-    "mps_set_profile",
+    "mps_set_profile", "mps_set_wait_limit",
     "mps_cell_order_noalloc", "mps_set_scenes", "mps_set_graph",
     "mps_gnn_create", "mps_gnn_use", "mps_gnn_train", "mps_gnn_params", "mps_gnn_state",
     "mps_gnn_features",
@@ -105,6 +105,7 @@ def load_library(path: str = LIB_PATH):
     lib.mps_set_field.argtypes = [P, C.c_char_p, DP]
     lib.mps_set_profile.argtypes = [P, C.c_int]
     lib.mps_set_graph.argtypes = [P, C.c_int]
+    lib.mps_set_wait_limit.argtypes = [P, C.c_uint]
     FP = C.POINTER(C.c_float)
     lib.mps_snapshot_vtu.argtypes = [P, C.c_char_p, C.c_int]
     lib.mps_wait_io.argtypes = [P]
@@ -342,6 +343,10 @@ class Solver:
 
     def get_state(self, *ptrs):
         return self._chk(self.lib.mps_get_state(self.h, *[p or None for p in ptrs]), "get_state")
+
+    def set_wait_limit(self, polls: int = 0):
+        """Bound of a grid wait of the one-launch solves, in polls (0: the default)."""
+        return self._chk(self.lib.mps_set_wait_limit(self.h, polls), "wait_limit")
 
     def set_profile(self, on: bool = True):
         return self._chk(self.lib.mps_set_profile(self.h, int(on)), "profile")

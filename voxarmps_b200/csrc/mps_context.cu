@@ -346,11 +346,12 @@ int allocate(mps_ctx* c)
     c->cg_part_cap = (size_t)5 * 8 * sms;
     TRY(dalloc(c, &c->cg_part, c->cg_part_cap));
     TRY(dalloc(c, &c->cg_scal, 32));
-    TRY(dalloc(c, &c->cg_flag, 4));
-    TRY(dalloc(c, &c->cg_bar, 4));
+    // the solve's flags and the one-launch solves' barrier words: one area, zeroed at once
+    TRY(dalloc(c, &c->cg_flag, kLoopWords));
+    c->cg_bar = reinterpret_cast<unsigned int*>(c->cg_flag + 4);
     TRY(dalloc(c, &c->d_err, 1));
     TRY(dalloc(c, &c->d_max, 1));
-    TRY(halloc(c, &c->cg_flag_host, 4));
+    TRY(halloc(c, &c->cg_flag_host, kLoopWords));
     TRY(halloc(c, &c->red_host, 32));
     TRY(halloc(c, &c->h_err, 1));
     // alternates of the persistent fields for the reorder (same order as
@@ -676,7 +677,7 @@ int mps_pressure(mps_ctx* c, int* iters, double* relres)
     }
     if (iters) *iters = c->cg_iters;
     if (relres) *relres = c->cg_relres;
-    return MPS_OK;
+    return c->cfg.method != 3 && c->cg_abandoned ? MPS_ERR_NOT_CONVERGED : MPS_OK;
 }
 
 // The stage sequence of one loop iteration (main.cu:1036-1337), enqueued
@@ -884,6 +885,15 @@ int mps_autotune(mps_ctx* c, int steps, mps_tuning* chosen)
     if (r != MPS_OK) return r;
     TRY(rp);
     if (chosen) *chosen = t;
+    return MPS_OK;
+}
+
+int mps_set_wait_limit(mps_ctx* c, unsigned int polls)
+{
+    if (!c) return MPS_ERR_ARG;
+    VMPS_CUDA(c, cudaSetDevice(c->device));
+    if (polls != c->loop_polls) drop_graphs(c);
+    c->loop_polls = polls;
     return MPS_OK;
 }
 

@@ -40,6 +40,8 @@ constexpr int kBlock = 256;
 // pass, formed against stored, 2D 1.9 k 3642 / 3926, 16 k 2369 / 2506, 29 k 1263 / 1297, 3D 24 k
 // 1816 / 1817, 54 k 897 / 887, 125 k 7030 / 6128, two-phase 86 k 5131 / 4987
 constexpr int kFormMax = 32768;
+// words of mps_ctx::cg_flag with cg_bar behind it; the one that a wait's failure sets
+constexpr int kLoopWords = 8, kLoopFailed = 5;
 
 // Cell grid of one support radius, NEIGHBOR's (functions.cu:2790-2802): x and
 // y cells of size re, z cells of size re + DELTA (3D).
@@ -154,6 +156,7 @@ struct mps_ctx {
     int cg_iters = 0;
     int cg_loop_kernels = 4, cg_nspmv = 0;
     bool cg_in_loop = false;  // the last solve ran in one cooperative launch
+    bool cg_abandoned = false;  // and a wait of its grid ran out
     bool ppe_pending = false;
     int ppe_warm = 1;  // initial guess of the last assembly (0: zero)
     // CUDA graph of one step per buffer parity (the reorder double-buffers
@@ -247,8 +250,11 @@ struct mps_ctx {
     size_t cg_part_cap = 0;      // doubles in cg_part
     double* cg_scal = nullptr;   // device scalars (rz, bb, rr, ...)
     double2* cg_zp = nullptr;    // k_cg_loop: (z, p) of every row
-    int* cg_flag = nullptr;      // [0] done, [1] iterations
-    unsigned int* cg_bar = nullptr;  // the one-launch solves' grid barrier: arrivals, monotonic per launch
+    int* cg_flag = nullptr;      // [0] done, [1] iterations, [3] refinements; then cg_bar
+    // the one-launch solves' grid barrier: [0] arrivals, monotonic per launch, [1] a
+    // wait ran out
+    unsigned int* cg_bar = nullptr;
+    unsigned loop_polls = 0;     // bound of a wait at it (0: the default)
     int* cg_flag_host = nullptr; // pinned
     double* red_host = nullptr;  // pinned scratch for scalars
     unsigned int* d_err = nullptr;

@@ -993,9 +993,11 @@ __global__ void k_ir_commit(double* scal, int* flag, double tol2, int use_cond,
 // residuals decide, as in the launches.
 //
 // Either has two grid-wide synchronisations per iteration.  Barriers: arrivals on one
-// counter that grows by the grid size per barrier; each wait is bounded (kBarPolls,
-// about a second and a half), past which the block sets MPS_ERR_NOT_CONVERGED and
-// leaves, so a lost block ends the solve instead of hanging the GPU.
+// counter that grows by the grid size per barrier; each wait is bounded (Loop::polls,
+// about a second and a half), past which the block sets MPS_ERR_NOT_CONVERGED and the
+// launch's word of failure, leaves its rows finite and clamped and returns, so a
+// lost block ends the solve instead of hanging the GPU and the solve reports
+// that it did not converge.
 constexpr int kLoopThreads = 1024;
 
 constexpr int kLoopMinRows = 64;    // rows per block at least (1.9 k rows: 32 rows 229 us per
@@ -1014,16 +1016,15 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p)
     return v;
 }
 
-constexpr unsigned kBarPolls = 1u << 21;
-
-// one thread's wait until `target` blocks have arrived; past the limit the failure goes
-// to the error word and to the block's *fail
-__device__ __forceinline__ void wait_arrivals(unsigned* bar, unsigned target, unsigned* err,
-                                              int* fail)
+// one thread's wait until `target` blocks have arrived at bar[0]; past the limit the
+// failure goes to the error word, to bar[1] and to the block's *fail
+__device__ __forceinline__ void wait_arrivals(unsigned* bar, unsigned target, unsigned polls,
+                                              unsigned* err, int* fail)
 {
     for (unsigned spins = 0; ld_acquire_u32(bar) < target;) {
-        if (++spins > kBarPolls) {
+        if (++spins > polls) {
             set_error(err, MPS_ERR_NOT_CONVERGED);
+            atomicExch(bar + 1, 1u);
             *fail = 1;
             break;
         }
@@ -1039,7 +1040,8 @@ struct Loop {
     double* part;
     double* scal;
     int* flag;
-    unsigned *bar, *err;
+    unsigned *bar, *err;  // bar: [0] arrivals, [1] a wait ran out
+    unsigned polls;       // bound of a wait
     double tol2;
     int maxit;
     int formed;       // r = b - A x0 is formed; x still holds the guess of every row
@@ -1201,7 +1203,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(Loop L)
         target += gridDim.x;
         if (threadIdx.x == 0) {
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(L.bar) : "memory");
-            wait_arrivals(L.bar, target, L.err, &s_fail);
+            wait_arrivals(L.bar, target, L.polls, L.err, &s_fail);
         }
         __syncthreads();
         return s_fail == 0;
@@ -1426,6 +1428,7 @@ struct Sync {
     unsigned* bar;
     unsigned* err;
     double* part;    // array q of block b at part[q * gridDim.x + b]
+    unsigned polls;
     unsigned target; // arrivals that complete the next barrier
     double (*warp)[32];
     double* tot;
@@ -1492,7 +1495,7 @@ struct Sync {
         __syncthreads();
         return *fail == 0;
     }
-    __device__ __forceinline__ void wait() { wait_arrivals(bar, target, err, fail); }
+    __device__ __forceinline__ void wait() { wait_arrivals(bar, target, polls, err, fail); }
 };
 
 // the block's k-th row: chunks of 32 rows dealt out to the blocks in turn
@@ -1540,7 +1543,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
     float *cd = reinterpret_cast<float*>(srow + R), *cr = cd + R, *cp = cr + R, *cs = cp + R,
           *cw = cs + R;
     if (threadIdx.x == 0) s_fail = 0;
-    Sync<ONE> sync{L.bar, L.err, L.part, 0u, s_warp, s_tot, &s_fail};
+    Sync<ONE> sync{L.bar, L.err, L.part, L.polls, 0u, s_warp, s_tot, &s_fail};
     // start: r32 = r, z = M^-1 r32, d = p = s = 0
     double v[4] = {0, 0, 0, 0};
     for (int k = threadIdx.x; k < nr; k += kLoopThreads) {
@@ -1571,12 +1574,12 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
         I.z[i] = z32;
         I.d[i] = 0.f;
     }
-    if (!sync.template sums<4>(v, 0)) return;
+    bool ok = sync.template sums<4>(v, 0);
     const double bb = v[0];
     double rr = v[1], rz = v[2], rin0 = v[3], rz_old = rz, alpha = 1.0;
     double eta2 = sweep_target(L.tol2, bb, rr);
     bool done = bb == 0.0 || rr <= L.tol2 * bb, first = true;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (ok && blockIdx.x == 0 && threadIdx.x == 0) {
         L.scal[S_BB] = bb;
         L.scal[S_RR0] = rr;
         L.scal[S_ZERO] = bb == 0.0 ? 1.0 : 0.0;
@@ -1584,7 +1587,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
     const Grp<G> q;
     const int grp = threadIdx.x / G;
     int it = 0, sweeps = 0;
-    while (!done) {
+    while (ok && !done) {
         // an inner iteration: w = A32 z and z.w
         double zw[1] = {0};
         for (int k = grp; k < nr; k += kLoopThreads / G) {
@@ -1596,7 +1599,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
                 zw[0] += (double)I.z[row(k)] * (double)wi;
             }
         }
-        if (!sync.template sums<1>(zw, 4)) return;
+        if (!(ok = sync.template sums<1>(zw, 4))) break;
         const double beta = first ? 0.0 : rz / rz_old;
         alpha = first ? rz / zw[0] : rz / (zw[0] - beta * rz / alpha);
         first = false;
@@ -1615,7 +1618,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
             v[0] += (double)r1 * (double)z1;
             v[1] += (double)r1 * (double)r1;
         }
-        if (!sync.template sums<2>(v, 5)) return;
+        if (!(ok = sync.template sums<2>(v, 5))) break;
         rz_old = rz;
         rz = v[0];
         const double rin = v[1];
@@ -1624,7 +1627,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
         // a refinement: r -= A64 d, x += d, and the next sweep's start
         for (int k = threadIdx.x; k < nr; k += kLoopThreads)
             if (srow[k].y >= 0) I.d[row(k)] = cd[k];
-        if (!sync.all()) return;
+        if (!(ok = sync.all())) break;
         v[0] = v[1] = v[2] = 0.0;
         for (int k = grp; k < nr; k += kLoopThreads / G) {
             const int2 m = srow[k];
@@ -1649,7 +1652,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
             v[1] += (double)r32 * (double)z32;
             v[2] += (double)r32 * (double)r32;
         }
-        if (!sync.template sums<3>(v, 7)) return;
+        if (!(ok = sync.template sums<3>(v, 7))) break;
         rr = v[0];
         rz = v[1];
         rin0 = v[2];
@@ -1668,7 +1671,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
                     L.sok[k] = (L.sbb[k] == 0.0 || acc <= L.tol2 * L.sbb[k]) ? 1 : 0;
                 }
             }
-            if (!sync.all()) return;
+            if (!(ok = sync.all())) break;
             bool all = true;
             for (int k = threadIdx.x; k < L.nscenes; k += kLoopThreads) all = all && __ldcg(L.sok + k) != 0;
             conv = __syncthreads_and(all) != 0;
@@ -1678,13 +1681,13 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_ir_loop(Loop L, IR I)
         eta2 = sweep_target(L.tol2, bb, rr);
         first = true;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (ok && blockIdx.x == 0 && threadIdx.x == 0) {
         L.scal[S_RR] = rr;
         L.flag[0] = 1;
         L.flag[1] = it;
         L.flag[3] = sweeps;
     }
-    loop_finish(L, sx, bb == 0.0);
+    loop_finish(L, sx, ok && bb == 0.0);
 }
 
 // y = A x on the unknown rows (0 elsewhere), with the last assembled matrix
@@ -1813,6 +1816,8 @@ constexpr int kLoopMaxBytes = 200 * 1024;
 // the virtual grid of a FP64 solve of up to kSmallRows rows is 4 blocks per SM, and no
 // more than the rows' groups fill (it sets the order of the sums, so it stays as it is)
 constexpr int kSmallRows = 16384, kSmallBps = 4;
+constexpr unsigned kBarPolls = 1u << 21;
+
 // blocks of the CG kernels' grid: blocks per SM from the autotuner, else as many as fit
 // (at most 8), fewer for small FP64 systems; cg_part holds [0,3*nblk) start/update
 // partials and [4*nblk,5*nblk) p.s.  whole: a whole warp per row (the slabs)
@@ -1910,6 +1915,7 @@ static int launch_loop(mps_ctx* c, const CG& A, const IR& I, double tol2, bool f
     L.flag = c->cg_flag;
     L.bar = c->cg_bar;
     L.err = c->d_err;
+    L.polls = c->loop_polls > 0 ? c->loop_polls : kBarPolls;
     L.tol2 = tol2;
     L.maxit = f.cg_max;
     L.formed = formed ? 1 : 0;
@@ -1928,7 +1934,9 @@ static int launch_loop(mps_ctx* c, const CG& A, const IR& I, double tol2, bool f
     L.srr = c->srr;
     L.sok = c->sok;
     L.nscenes = c->nscenes;
-    if (!one) VMPS_CUDA(c, cudaMemsetAsync(c->cg_bar, 0, sizeof(unsigned), c->stream));
+    // an abandoned solve leaves the outcome of no earlier one
+    if (!one)
+        VMPS_CUDA(c, cudaMemsetAsync(c->cg_flag, 0, kLoopWords * sizeof(int), c->stream));
     IR i = I;
     void* cg_args[] = {&L};
     void* ir_args[] = {&L, &i};
@@ -2119,7 +2127,7 @@ int vmps_ppe(mps_ctx* c, bool report)
         vmps_count_launch(1);
     }
     if (report) {
-        VMPS_CUDA(c, cudaMemcpyAsync(c->cg_flag_host, c->cg_flag, 4 * sizeof(int),
+        VMPS_CUDA(c, cudaMemcpyAsync(c->cg_flag_host, c->cg_flag, kLoopWords * sizeof(int),
                                      cudaMemcpyDeviceToHost, st));
         VMPS_CUDA(c, cudaMemcpyAsync(c->red_host, c->cg_scal, S_COUNT * sizeof(double),
                                      cudaMemcpyDeviceToHost, st));
@@ -2140,7 +2148,7 @@ __global__ void k_report(unsigned int* err, unsigned int* h_err, const int* __re
         *h_err = *err;
         *err = 0;
     }
-    if (t < 4) h_flag[t] = flag[t];
+    if (t < kLoopWords) h_flag[t] = flag[t];
     if (t < S_COUNT) h_scal[t] = scal[t];
 }
 
@@ -2175,6 +2183,9 @@ int vmps_ppe_finish(mps_ctx* c)
     c->cg_relres = bb > 0 ? sqrt(rr / bb) : 0.0;
     c->cg_r0 = bb > 0 ? sqrt(c->red_host[S_RR0] / bb) : 0.0;
     if (c->nscenes > 1) c->cg_relres = c->red_host[S_WORST];
+    // a one-launch solve whose grid wait ran out: no residual to report
+    c->cg_abandoned = c->cg_in_loop && c->n > kLoopOneBlock && c->cg_flag_host[kLoopFailed] != 0;
+    if (c->cg_abandoned) c->cg_relres = NAN;
     if (!(c->cg_relres <= f.cg_tol)) c->host_err |= MPS_ERR_NOT_CONVERGED;
     VMPS_CUDA(c, cudaGetLastError());
     return MPS_OK;
