@@ -49,12 +49,15 @@ def _check(s):
     assert not p[s.get("bcon") != 0].any()
 
 
+MAKE = {"dam": _dam, "batch": _batch}
+
+
 @pytest.mark.parametrize("graph", [False, True])
 @pytest.mark.parametrize("make, opts", [
-    (_dam, dict()), (_dam, dict(warm_start=0)), (_dam, dict(precision=1)),
-    (_batch, dict(precision=1))], ids=str)
+    ("dam", dict()), ("dam", dict(warm_start=0)), ("dam", dict(precision=1)),
+    ("batch", dict(precision=1))], ids=str)
 def test_step(make, opts, graph):
-    s = _solver(*make(**opts))
+    s = _solver(*MAKE[make](**opts))
     s.set_graph(graph)
     for _ in range(2):  # both buffer sets
         assert s.step() == 0
