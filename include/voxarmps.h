@@ -223,7 +223,8 @@ int mps_set_wait_limit(mps_ctx* ctx, unsigned int polls);
  * small_lanes: lanes per row of the PND-radius list in the list build and
  * every stage over that list (4 or 8; sums over a row
  * change order with it, results stay within rounding).  cg_blocks_per_sm:
- * grid of the CG kernels (1..8, 0 = as many as fit). */
+ * grid of the CG kernels (1..8, 0 = as many as fit); it sets the order of
+ * the solve's sums, and where the solve is one launch nothing else. */
 typedef struct mps_tuning {
     int small_lanes;
     int cg_blocks_per_sm;
@@ -232,7 +233,9 @@ int mps_get_tuning(mps_ctx* ctx, mps_tuning* out);
 int mps_set_tuning(mps_ctx* ctx, const mps_tuning* in);
 /* Time every candidate over `steps` steps each (CUDA events, eager launches;
  * these are real steps that advance the simulation), keep the fastest per
- * parameter and return it.  Call it in place of the first warm-up steps. */
+ * parameter and return it.  Where the pressure solve is one launch
+ * cg_blocks_per_sm is not searched: it keeps its value (8 when unset).  Call
+ * it in place of the first warm-up steps. */
 int mps_autotune(mps_ctx* ctx, int steps, mps_tuning* chosen);
 
 /* ---- learned CG initial guess (no reference counterpart) ---------------- *

@@ -833,7 +833,11 @@ static int autotune_search(mps_ctx* c, int steps, mps_tuning& t)
         *rest = median(b);
         return MPS_OK;
     };
-    if (c->cfg.method != 3) {
+    if (vmps_one_launch(c)) {
+        // the solve's grid is its own there: nothing to time, as many as fit
+        if (t.cg_blocks_per_sm == 0) t.cg_blocks_per_sm = 8;
+        TRY(mps_set_tuning(c, &t));
+    } else if (c->cfg.method != 3) {
         int best = t.cg_blocks_per_sm;
         double best_ms = 1e300;
         for (int bps : {1, 2, 4, 8}) {
@@ -866,7 +870,8 @@ static int autotune_search(mps_ctx* c, int steps, mps_tuning& t)
     return mps_set_tuning(c, &t);
 }
 
-// Coordinate search: the CG grid by the PPE time per CG iteration, then the
+// Coordinate search: the CG grid by the PPE time per CG iteration (where the
+// solve takes more than one launch), then the
 // PND-radius lane width by the time of the rest of the step.  Each candidate
 // runs `steps` profiled steps; the median step decides.  On failure the
 // previous tuning and profiling state are restored.

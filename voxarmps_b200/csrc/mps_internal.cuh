@@ -530,6 +530,8 @@ int vmps_pressure_wc(mps_ctx* ctx);
 // report: copy the outcome to the host (a step's last launch does it there)
 int vmps_ppe(mps_ctx* ctx, bool report = true);
 int vmps_report(mps_ctx* ctx);
+// whether a pressure solve of this context runs in one cooperative launch
+bool vmps_one_launch(mps_ctx* ctx);
 int vmps_ppe_finish(mps_ctx* ctx);
 int vmps_ppe_apply(mps_ctx* ctx, const double* x, double* y);
 int vmps_gnn_guess(mps_ctx* ctx);

@@ -1868,10 +1868,10 @@ static LoopShape loop_shape(const mps_ctx* c, int sms, int nparts)
     return s;
 }
 
-static bool use_cg_loop(mps_ctx* c)
+bool vmps_one_launch(mps_ctx* c)
 {
     const bool mixed = c->cfg.precision >= 1;
-    if ((!mixed && c->nscenes > 1) || c->n > (mixed ? kIrLoopMax : kLoopMax))
+    if (c->cfg.method == 3 || (!mixed && c->nscenes > 1) || c->n > (mixed ? kIrLoopMax : kLoopMax))
         return false;
     // mixed precision: the launch's sums and recurrence are its own, and a
     // non-Newtonian scene magnifies any difference of rounding
@@ -1960,7 +1960,7 @@ int vmps_ppe(mps_ctx* c, bool report)
     bool fused = false;
     // the whole solve in one cooperative launch; a profiled FP64 solve, whose
     // products are timed, takes the launches, with the same bits
-    const bool loop = use_cg_loop(c) && (mixed || !c->profile);
+    const bool loop = vmps_one_launch(c) && (mixed || !c->profile);
     const bool narrow = n <= kNarrowMaxRows;  // 16 lanes per row in the FP64 products
     {
         int r = ppe_assemble(c, &warm, c->cg_r, &fused);
