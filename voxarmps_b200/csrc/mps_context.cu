@@ -1137,6 +1137,7 @@ int mps_step_io(mps_ctx* c, const double* const* in, double* const* out)
     if (r & (MPS_ERR_ARG | MPS_ERR_CUDA)) {
         // the step stopped before taking the fields: leave no copy pending
         cudaStreamSynchronize(c->stream_io);
+        cudaStreamSynchronize(c->stream);
         return r;
     }
     return r | mps_get_state(c, out[0], out[1], out[2], out[3], out[4], out[5], out[6]);
