@@ -1176,7 +1176,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(Loop L)
     double* const part = ONE ? s_part : L.part;
     double* const prod = ONE ? s_prod : L.s;
     double2* const zp = ONE ? s_zp : L.zp;
-    auto read = [](const double* a) { return ONE ? *a : __ldcg(a); };
+    auto read = [](const double* a) { return ONE ? *a : __ldcg(a); };  // (of another block)
     const Virtual vec = virtual_grid(A.n, nv, kRedThreads, gridDim.x);
     const Virtual pro = virtual_grid(A.n, nv, GV, gridDim.x);
     const int t = threadIdx.x & (kRedThreads - 1), h = threadIdx.x / kRedThreads;
@@ -1211,6 +1211,16 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(Loop L)
     // the sums of `all` virtual blocks in the arrays first, first + 1, ..., added in
     // reduce_parts' order; total j goes to done(j, total) in one thread
     auto totals = [&](int count, int all, int first, auto done) {
+        if (ONE) {  // at most 32 virtual blocks: the first warp's part of that order
+            const int j = threadIdx.x >> 5;
+            if (j < count) {
+                double v = lane < all ? part[(first + j) * pitch + lane] : 0.0;
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+                if (lane == 0) done(j, 0.0 + v);
+            }
+            __syncthreads();
+            return;
+        }
         if (h < count) {
             const double* sums = part + (first + h) * pitch;
             double v = 0.0;
