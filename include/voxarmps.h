@@ -213,7 +213,7 @@ int mps_set_profile(mps_ctx* ctx, int on);
  * identical to eager mode.  Off while profiling (mps_set_profile). */
 int mps_set_graph(mps_ctx* ctx, int on);
 /* Bound of a wait of the one-launch pressure solves' grid, in polls of its
- * counter (0, the default: 2^21, about a second and a half).  A solve whose
+ * counter (0, the default: 2^23, about a second and a half).  A solve whose
  * wait runs out is abandoned: the pressures are clamped and finite,
  * cg_relres is NaN, cg_iters 0, MPS_ERR_NOT_CONVERGED is set, and
  * mps_pressure returns it. */

@@ -994,7 +994,7 @@ __global__ void k_ir_commit(double* scal, int* flag, double tol2, int use_cond,
 //
 // Either has two grid-wide synchronisations per iteration.  Barriers: arrivals on one
 // counter that grows by the grid size per barrier; each wait is bounded (Loop::polls,
-// about a second and a half), past which the block sets MPS_ERR_NOT_CONVERGED and the
+// about a second and a half by default), past which the block sets MPS_ERR_NOT_CONVERGED and the
 // launch's word of failure, leaves its rows finite and clamped and returns, so a
 // lost block ends the solve instead of hanging the GPU and the solve reports
 // that it did not converge.
@@ -1826,7 +1826,7 @@ constexpr int kLoopMaxBytes = 200 * 1024;
 // the virtual grid of a FP64 solve of up to kSmallRows rows is 4 blocks per SM, and no
 // more than the rows' groups fill (it sets the order of the sums, so it stays as it is)
 constexpr int kSmallRows = 16384, kSmallBps = 4;
-constexpr unsigned kBarPolls = 1u << 21;
+constexpr unsigned kBarPolls = 1u << 23;  // of 160 to 175 ns
 
 // blocks of the CG kernels' grid: blocks per SM from the autotuner, else as many as fit
 // (at most 8), fewer for small FP64 systems; cg_part holds [0,3*nblk) start/update
