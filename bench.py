@@ -428,6 +428,10 @@ def run_ours(args):
     prof_ms = rank_max(p0.elapsed_time(p1))
     spmv_ms = s.scalar("spmv_ms")
     spmv_n = s.scalar("spmv_launches")
+    # a mixed solve in one launch stays so when profiled (an FP64 one takes the launches):
+    # the product is then a part of the launch, its matrix comes out of L2, and the
+    # figures are per iteration
+    looped = bool(s.scalar("one_launch_solve"))
     nnz_a = s.scalar("nnz_a")
     rows = float((s.get("bcon") == 0).sum())
     # ---- end-to-end through the API with host buffers ----
@@ -460,12 +464,12 @@ def run_ours(args):
     spmv_kernel = ("k_ir_spmv (mixed PPE: FP32 inner SpMV + FP64 refinement, CSR, warp per row)"
                    if mixed else "k_cg_spmv (PPE SpMV, FP64 CSR, warp per row)")
     spmv_source = f"CUDA events around every {name} launch over the K profiled steps"
-    if s.scalar("one_launch_solve"):  # the product is a part of the launch: per iteration
-        name = "k_ir_loop" if mixed else "k_cg_loop"
-        spmv_kernel = (f"{name} (whole solve in one launch; per iteration: product, vector "
+    if looped:
+        spmv_kernel = ("k_ir_loop (whole solve in one launch; per iteration: product, vector "
                        "updates and two grid synchronisations)")
-        spmv_source = (f"CUDA events around every {name} launch over the K profiled steps, "
+        spmv_source = ("CUDA events around every k_ir_loop launch over the K profiled steps, "
                        "divided by its iterations")
+    unit = "iteration" if looped else "launch"
     # DRAM bytes per launch from the ncu capture of the FP64 SpMV (scaled by
     # its traffic/algorithmic ratio); not captured for the mixed kernel
     traffic = None if mixed else SPMV_TRAFFIC_OVER_ALGORITHMIC * algo
@@ -531,12 +535,13 @@ def run_ours(args):
             "cg_relres_last": relres, "status_bits": status,
             "stage_ms": {k[3:]: statistics.mean(v) for k, v in stage.items()},
             "roofline": {"kernel": spmv_kernel,
-                         "bound": "hbm",
+                         "bound": "l2 and grid synchronisation" if looped else "hbm",
                          "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": (achieved / peak) if achieved else None,
                          "traffic": traffic, "peak_source": peak_kind,
-                         "algorithmic_bytes_per_launch": algo,
-                         "avg_launch_ms": spmv_avg_ms, "launches_timed": int(spmv_n),
+                         f"algorithmic_bytes_per_{unit}": algo,
+                         f"avg_{unit}_ms": spmv_avg_ms,
+                         "iterations_timed" if looped else "launches_timed": int(spmv_n),
                          "duration_source": spmv_source},
             "e2e": {"value": whole_job_rate(n_job * args.steps, 1, e2e_ms), "unit": METRIC,
                     "h2d_bytes_per_step": bytes_state, "d2h_bytes_per_step": bytes_state},

@@ -329,9 +329,9 @@ __global__ void k_scene_ranges(int n, const int* __restrict__ scene, int* __rest
 // of x.  Rows are stored in scan order (y, z outer, memory order inside);
 // the reference's own order (x offset outermost, ascending id per cell) is
 // restored when lists are exported (mps_download_lists).
-// 6 resident blocks per SM (40 registers): with the warp's groups stepping
-// together, the neighbour stage 4.51 ms on the 1.6 M-particle dam against
-// 4.61 ms at 8 blocks (32 registers, spills) and 4.69 ms for divergent groups
+// 6 resident blocks per SM (40 registers).  Both lists, us, at 4 / 6 / 8 blocks (32
+// registers, spills): 3D, 54 k particles 142 / 148 / 159; 2D, 345 k 159 / 151 / 149, 1.9 k
+// 20 / 20 / 23
 template <int DIM, int G, bool PERM>
 __global__ void __launch_bounds__(256, 6) k_lists(int n, Grid g, double cut, float cut_lo, float cut_hi, int cap,
                         const double4* __restrict__ P4, const float4* __restrict__ P4f,
@@ -485,8 +485,9 @@ __global__ void __launch_bounds__(256, 6) k_lists(int n, Grid g, double cut, flo
 // Rows are stored in scan order (y, z outer, memory order inside); the
 // reference's own order (x offset outermost, ascending id per cell) is
 // restored when lists are exported (mps_download_lists).
-// entries a lane may hold back: with 48, 32 blocks (warps) fit an SM (1.6 M dam,
-// Laplacian and PND list 1328 / 524 us; 56 entries 1372 / 527, 64 entries 1419 / 545)
+// entries a lane may hold back: with 48 a block takes 7.1 KB of shared memory and 1 KB
+// reserved, and 28 blocks (warps) fit an SM (1.6 M dam, Laplacian and PND list 1328 /
+// 524 us; 56 entries, 24 blocks, 1372 / 527; 64 entries, 22 blocks, 1419 / 545)
 constexpr int kListBuf = 48;
 constexpr int kListFlush = kListBuf - 32;  // flushed once a lane holds more (32 candidates add at most 32)
 // cells a warp's particles may span along x in one pass: a sparse row's next

@@ -33,11 +33,10 @@ constexpr int kRedThreads = 256;
 // warp per row (16 or 8 lanes: 0.69 ms against 0.61 ms per launch); the
 // assembly runs 16 lanes per row (PPE stage 12.4 ms against 12.8 ms at 32)
 constexpr int kRowG = 32;
-// systems of at most this many rows run their FP64 products with 16 lanes per
-// row (two rows per warp) where they take one launch per kernel (FP64 batches, the
-// start from other guesses): 86,118 rows of ~50 entries 2.04 against 2.38 ms per
-// step with whole warps; the 1.6 M-particle dam keeps whole warps (0.61 against 0.69
-// ms per SpMV)
+// systems of at most this many rows sum their FP64 products over 16 lanes per row
+// (two rows per warp in the launches; k_cg_loop sums in the same order): 86,118 rows of
+// ~50 entries 2.04 against 2.38 ms per step with whole warps; the 1.6 M-particle dam
+// keeps whole warps (0.61 against 0.69 ms per SpMV)
 constexpr int kNarrowMaxRows = 262144;
 constexpr int kAsmG = 16;
 // lanes per row of the mixed-precision products (inner FP32 and refinement):
@@ -992,19 +991,19 @@ __global__ void k_ir_commit(double* scal, int* flag, double tol2, int use_cond,
 // arithmetic the iterates are the textbook form's; the refinements' FP64
 // residuals decide, as in the launches.
 //
-// Either has two grid-wide synchronisations per iteration.  Barriers: arrivals on one
-// counter that grows by the grid size per barrier; each wait is bounded (Loop::polls,
-// about a second and a half by default), past which the block sets MPS_ERR_NOT_CONVERGED and the
-// launch's word of failure, leaves its rows finite and clamped and returns, so a
-// lost block ends the solve instead of hanging the GPU and the solve reports
-// that it did not converge.
+// Two grid-wide synchronisations per iteration (FP64 with p stored: three).
+// Barriers: arrivals on one counter that grows by the grid size per barrier; each
+// wait is bounded (Loop::polls, about a second and a half by default), past which the
+// block sets MPS_ERR_NOT_CONVERGED and the launch's word of failure, leaves its rows
+// finite and clamped and returns, so a lost block ends the solve instead of hanging
+// the GPU and the solve reports that it did not converge.
 constexpr int kLoopThreads = 1024;
 
-constexpr int kLoopMinRows = 64;    // rows per block at least (1.9 k rows: 32 rows 229 us per
-                                    // step, 64 227, 128 234, 256 249)
+constexpr int kLoopMinRows = 64;    // rows per block at least (us per step with 32 / 64 / 128:
+                                    // 1.9 k rows 182 / 182 / 198, 8.3 k 201 / 202 / 217)
 // scenes of up to this many particles solve in one block, without a grid-wide
-// synchronisation (a step from host arrays of 336 particles 239 -> 209 us; 663 particles
-// 171 us per step in one block or several, 1,093 235 against 182)
+// synchronisation (us per step in one block against several: 200 particles 119 / 144, 336
+// 130 / 162, 408 234 / 244, 483 162 / 168, 512 280 / 274)
 constexpr int kLoopOneBlock = 512;
 // shared memory per row of the mixed solve: three doubles, (offset, length), five floats
 constexpr int kIrLoopRow = 3 * 8 + 8 + 5 * 4;
@@ -1156,9 +1155,9 @@ __device__ __forceinline__ double spmv_row_of(const CG& A, const Grp<G>& q, cons
 //
 // G lanes per row: 16; in 2D (about 40 entries a row) 8 when p is stored or the grid is one
 // block (165 k rows 1801 us per pass against 1880; 1.9 k rows 4222 against 3926).
-// Bound by the exchanges in small scenes (1.9 k rows: 13,000 of 15,000 cycles per
-// iteration), by the matrix stream from L2 in large ones (two-phase scene, 86 k rows:
-// 24.6 us per iteration against 37.7 in four launches).
+// Bound by the exchanges in small scenes (1.9 k rows: 9,300 of 13,300 cycles per
+// iteration), by the matrix stream from L2 in large ones (two-phase scene, 86 k rows: the
+// product 15,500 of 33,600 cycles; 17 us per iteration against 29 in four launches).
 template <int G, bool ONE, bool STORE>
 __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(Loop L)
 {
@@ -2209,7 +2208,8 @@ int vmps_ppe_finish(mps_ctx* c)
 // order over the blocks); the caller adds them over the ranks, forms alpha
 // and beta, and between the calls exchanges the ghost entries of the CG
 // vectors (mps_get_rows / mps_set_rows on "pnew" and "cg_p").  With one
-// context the sequence reproduces vmps_ppe's FP64 Jacobi-PCG.
+// context the sequence is vmps_ppe's FP64 Jacobi-PCG with every product summed by a
+// whole warp (vmps_ppe sums by half ones up to kNarrowMaxRows rows).
 namespace {
 
 __global__ void k_local_sums(int nparts, int count, const double* __restrict__ part,

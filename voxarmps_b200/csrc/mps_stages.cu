@@ -388,8 +388,8 @@ __global__ void __launch_bounds__(256, 6) k_predict_p(int n, Lists Ls, PredArgs 
     if (DIM == 3) pz[I] = pc * sum3;
 }
 
-// lanes per particle of the FP32 viscous sums (measured: 8 lanes 3.9 ms of
-// explicit stages on the 1.6 M-particle dam, 16 lanes 4.1, a warp 4.4)
+// lanes per particle of the FP32 viscous sums (explicit stages of the 1.6 M-particle
+// dam: 4 lanes 1.97 ms, 8 1.99, 16 2.17, a warp 2.48)
 constexpr int kPred32G = 8;
 // Mixed precision: the viscous Laplacian's neighbour sums in FP32 (FP32
 // positions relative to the box, FP32 velocities, FP32 weights and sums);
@@ -397,8 +397,9 @@ constexpr int kPred32G = 8;
 // TURB: the eddy-viscosity sums (sum7..9, times neut) are kept only with
 // SPS on; without it neut is 0 and they add nothing.
 template <int DIM, bool TURB, int KT, bool BYKIND>
-// 4 blocks per SM: the two-entries-in-flight loop needs the registers
-// (measured 4.4 ms explicit stages on the 1.6 M dam against 5.1 at 5 blocks)
+// 4 blocks per SM, which the general kernel function's registers once needed; with its
+// type known at compile time 5 blocks measure better (explicit stages of the 1.6 M dam
+// 1.99 ms at 4, 1.73 ms at 5)
 __global__ void __launch_bounds__(256, 4)
 k_predict32(int n, Lists Ll, PredArgs A, WKf wl, const double* __restrict__ meu,
             const double4* __restrict__ P4, const double4* __restrict__ U4,
@@ -501,8 +502,8 @@ k_predict32(int n, Lists Ll, PredArgs A, WKf wl, const double* __restrict__ meu,
 
 // PREDICTION, second part: viscous Laplacian over the Laplacian list, one
 // group of kPredG lanes per particle, then u* and x*.
-// lanes per particle of the viscous sums: 8 (explicit stages 5.0 ms on the
-// 1.6 M-particle dam against 5.5 ms with a whole warp; 4 is no better)
+// lanes per particle of the viscous sums: 8 (explicit stages of the 1.6 M-particle
+// dam: 4 lanes 2.60 ms, 8 2.54, 16 2.64, a warp 2.92)
 // 128 threads at 72 registers (7 blocks, 28 warps per SM): the two entries in
 // flight need them (256 threads at 64 registers spill: 507 against 497 us)
 constexpr int kPredThreads = 128;
